@@ -310,6 +310,7 @@ void fill_args( rgdn_stream* s, uint32_t fi, const rgdn_frame_params* p, FrameAr
     u.niter             = p->atrousIterations == 0 ? 4u : p->atrousIterations;
     u.flags             = p->flags;
     u.frameId           = p->frameId;
+    u.prefetchRows      = u.W * u.H >= PREFETCH_MIN_PIXELS ? ( PREFETCH_PIXELS + u.W - 1 ) / u.W : 0;
 
     const uint32_t pf = fi ^ 1u;
 #define CUR( fb ) ( (void*)plane_ptr_mut( s, fb, fi ) )

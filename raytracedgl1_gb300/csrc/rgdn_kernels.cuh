@@ -339,6 +339,11 @@ template< bool BF > struct Sto16
 };
 template<> struct Sto< MODE_F16 > : Sto16< false > {};
 template<> struct Sto< MODE_BF16 > : Sto16< true > {};
+// texel bytes: colour + variance and history length, colour, moments
+template< int M > struct TexelBytes
+{
+    static constexpr int cv = M == MODE_F32 ? 16 : 8, colour = M == MODE_REF ? 4 : M == MODE_F32 ? 16 : 8, moments = M == MODE_REF ? 4 : 8;
+};
 
 // zero-texel-outside-the-image loads of the mode-dependent images
 template< int M > __device__ __forceinline__ float3 ld3z( const FrameArgs& a, const void* p, int x, int y )
@@ -784,6 +789,41 @@ __device__ __forceinline__ void fill_u8( float* u8, int t )
 // before the first global-memory access. Without a programmatic dependency both are no-ops.
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile( "griddepcontrol.launch_dependents;" ::: "memory" ); }
 __device__ __forceinline__ void pdl_wait() { asm volatile( "griddepcontrol.wait;" ::: "memory" ); }
+
+// L2 prefetch of the rows that the blocks some way ahead in launch order will read. The passes
+// are bound by the latency of loads: once a frame's planes no longer fit the 129 MB L2, each
+// block's first reads of a row go to DRAM. One block in 8 asks for 256 columns of those rows
+// ahead of time, with one bulk prefetch per plane and row (cp.async.bulk.prefetch.L2): no register
+// holds it and it takes next to no issue slots. On GB300 at 1920x1080 fp16 the temporal pass went
+// from 99.3 to 91.8 us, the a-trous iterations from 59.4 / 51.7-52.7 / 73.7 to 55.2 / 51.4-51.6 /
+// 71.7, and the step from 457 to 441 us; at 3840x2160 bf16 372.9 to 340.5, 224.9 / 193-195 / 278.9
+// to 208.8 / 188-191 / 267.9, anti-firefly 126.3 to 122.6, and the step from 1747 to 1672 us.
+//
+// The variance pass reads what the two passes before it wrote and measured 3 % slower with it.
+// bytes [b0, b1) of p: the whole 16-byte units among them
+__device__ __forceinline__ void prefetch_bytes( const void* p, size_t b0, size_t b1 )
+{
+    b0               = ( b0 + 15 ) & ~(size_t)15;
+    const int      n = (int)( ( b1 & ~(size_t)15 ) - b0 );
+    const uint8_t* q = static_cast< const uint8_t* >( p ) + b0;
+    if( n > 0 ) asm volatile( "cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"( __cvta_generic_to_global( q ) ), "r"( n ) : "memory" );
+}
+// N planes, TH rows per tile of 32 columns; plane( k, p, texelBytes ) gives plane k. The first row is
+// Uniform::prefetchRows and `ahead` rows below the tile's. The kernels that call it (PF) are builds of
+// their own, launched where prefetchRows is not 0: even an untaken branch in the others cost small
+// frames 0.5-1 %.
+template< int N, int TH, class Plane > __device__ __forceinline__ void prefetch_ahead( const Uniform& u, const int t, const int ahead, Plane plane )
+{
+    if( ( blockIdx.x & 7 ) != 0 || t >= N * TH ) return;
+    const int y = blockIdx.y * TH + u.prefetchRows + ahead + t % TH;
+    if( y >= u.H ) return;
+    const int    x0 = blockIdx.x * 32;
+    const size_t c0 = (size_t)y * u.W + x0, c1 = c0 + min( 256, u.W - x0 );
+    const void*  p  = nullptr;
+    int          e  = 0;
+    plane( t / TH, p, e );
+    if( p ) prefetch_bytes( p, c0 * e, c1 * e );
+}
 
 // Tile functions: one thread per pixel (or stratum) of the blockDim-sized tile (bx, by) of
 // frame `a`. The single-frame kernels run one tile per block; the batched kernels loop a
@@ -1296,7 +1336,7 @@ __device__ __forceinline__ void temporal_tile( const FrameArgs& a, int bx, int b
 // but the filtered gradient is read before this grid waits for the chain, so the reprojection
 // and the taps overlap the chain's last kernels. The gradient chain writes nothing else this
 // pass reads, and reads nothing this pass writes.
-template< int M, bool FAST, bool GEOM, bool GEOMPREV, int NT = 256, int MINB = 1, bool EARLY = false >
+template< int M, bool FAST, bool GEOM, bool GEOMPREV, int NT = 256, int MINB = 1, bool EARLY = false, bool PF = false >
 __global__ void __launch_bounds__( NT, MINB ) k_temporal( const FrameArgs a )
 {
     __shared__ float u8[ 256 ];
@@ -1304,6 +1344,29 @@ __global__ void __launch_bounds__( NT, MINB ) k_temporal( const FrameArgs a )
     for( int k = threadIdx.y * blockDim.x + threadIdx.x; k < 256; k += NT ) fill_u8( u8, k );
     if( !EARLY ) pdl_wait();
     __syncthreads();
+    if constexpr( PF )
+        prefetch_ahead< 16, NT / 32 >( a.u, threadIdx.y * 32 + threadIdx.x, 0, [ & ]( int k, const void*& p, int& e ) {
+            using B = TexelBytes< M >;
+            switch( k )
+            {
+                case 0: p = GEOMPREV ? a.geomPrev : nullptr, e = 16; break;
+                case 1: p = a.surfPos, e = 16; break;
+                case 2: p = a.surfPosPrev, e = 16; break;
+                case 3: p = a.motion, e = 8; break;
+                case 4: p = a.viewDir, e = 8; break;
+                case 5: p = a.unfD, e = 4; break;
+                case 6: p = a.unfS, e = 4; break;
+                case 7: p = a.unfI, e = 4; break;
+                case 8: p = a.normal, e = 4; break;
+                case 9: p = a.diffHistory, e = B::cv; break;
+                case 10: p = a.momentsPrev, e = B::moments; break;
+                case 11: p = a.histLenPrev, e = B::cv; break;
+                case 12: p = a.specAccumPrev, e = B::colour; break;
+                case 13: p = a.indirAccumPrev, e = B::colour; break;
+                case 14: p = a.depth, e = 2; break;
+                default: p = a.mr, e = 2; break;
+            }
+        } );
     temporal_tile< M, FAST, GEOM, GEOMPREV, EARLY >( a, blockIdx.x, blockIdx.y, u8 );
 }
 
@@ -1685,11 +1748,16 @@ template< int M > __device__ __forceinline__ void antifirefly_fast_tile( const F
     }
 }
 
-template< int M > __global__ void __launch_bounds__( 256, ( M == MODE_F16 || M == MODE_BF16 ) ? 4 : 3 ) k_antifirefly_fast( const FrameArgs a )
+template< int M, bool PF > __global__ void __launch_bounds__( 256, ( M == MODE_F16 || M == MODE_BF16 ) ? 4 : 3 ) k_antifirefly_fast( const FrameArgs a )
 {
     __shared__ AfShared< M > sh;
     pdl_launch_dependents();
     pdl_wait();
+    if constexpr( PF )
+        prefetch_ahead< 3, 32 >( a.u, threadIdx.y * 32 + threadIdx.x, 2, [ & ]( int k, const void*& p, int& e ) {
+            p = k == 0 ? a.diffTemp : k == 1 ? a.specAccum : a.indirAccum;
+            e = TexelBytes< M >::colour;
+        } );
     antifirefly_fast_tile< M >( a, blockIdx.x, blockIdx.y, sh );
 }
 
@@ -2297,7 +2365,7 @@ __device__ __forceinline__ void atrous_tile( const FrameArgs& a, const int iter,
 // NT threads per block (32 x NT/32 tiles), MINB resident blocks per SM. ITER >= 0 builds the
 // kernel for that iteration (the argument `iter` is then ITER): the step is a constant, so the
 // taps of a stencil row share one address and differ by immediate offsets.
-template< int M, bool FAST, bool HIST, bool GEOMIN, int NT = 256, int MINB = 3, int ITER = -1 >
+template< int M, bool FAST, bool HIST, bool GEOMIN, int NT = 256, int MINB = 3, int ITER = -1, bool PF = false >
 __global__ void __launch_bounds__( NT, MINB ) k_atrous( const FrameArgs a, const int iterArg )
 {
     const int iter = ITER >= 0 ? ITER : iterArg;
@@ -2313,6 +2381,19 @@ __global__ void __launch_bounds__( NT, MINB ) k_atrous( const FrameArgs a, const
     }
     pdl_wait();
     __syncthreads();
+    if constexpr( PF )
+    {
+        const AtrousIO io = atrous_io< M >( a, iter );
+        prefetch_ahead< 6, NT / 32 >( a.u, t, 1 << iter, [ & ]( int k, const void*& p, int& e ) {
+            using B = TexelBytes< M >;
+            if( k == 0 ) p = a.geom, e = 16;
+            else if( k == 1 ) p = io.diffSrc, e = B::cv;
+            else if( k == 2 ) p = io.specSrc, e = B::colour;
+            else if( k == 3 ) p = io.indirSrc, e = B::colour;
+            else if( k == 4 ) p = a.histLen, e = B::cv;
+            else if( Sto< M >::varPlane ) p = io.varSrc, e = 4;
+        } );
+    }
     atrous_tile< M, FAST, HIST, GEOMIN >( a, iter, blockIdx.x, blockIdx.y, u8, hist );
     if( HIST )
     {
@@ -3953,6 +4034,7 @@ template< int M > cudaError_t launch_stage_t( const FrameArgs& a, int stage, int
     const dim3 blk( 32, 8 );
     const dim3 grid( ( a.u.W + 31 ) / 32, ( a.u.H + 7 ) / 8 );
     const dim3 gridG( ( a.u.GW + 31 ) / 32, ( a.u.GH + 7 ) / 8 );
+    const dim3 tgrid( grid.x, ( a.u.H + 3 ) / 4 );
     switch( stage )
     {
         case RGDN_STAGE_GRADIENT_SAMPLES: e = launch_pdl( dev::k_gradient_samples< M >, gridG, blk, 0, s, a, a.disPing ); break;
@@ -3961,19 +4043,19 @@ template< int M > cudaError_t launch_stage_t( const FrameArgs& a, int stage, int
         case KF_TEMPORAL_EXACT_GEOM: e = launch_pdl( dev::k_temporal< M, false, true, false >, grid, blk, 0, s, a ); break;
         case KF_TEMPORAL_EXACT_GEOM_GP: e = launch_pdl( dev::k_temporal< M, false, true, true >, grid, blk, 0, s, a ); break;
         case KF_TEMPORAL_FAST:
-            e = launch_pdl( dev::k_temporal< M, true, true, false, 128, 8 >, dim3( grid.x, ( a.u.H + 3 ) / 4 ), dim3( 32, 4 ), 0, s, a );
+            e = launch_pdl( a.u.prefetchRows ? dev::k_temporal< M, true, true, false, 128, 8, false, true > : dev::k_temporal< M, true, true, false, 128, 8 >, tgrid, dim3( 32, 4 ), 0, s, a );
             break;
         case KF_TEMPORAL_FAST_GP:
-            e = launch_pdl( dev::k_temporal< M, true, true, true, 128, 8 >, dim3( grid.x, ( a.u.H + 3 ) / 4 ), dim3( 32, 4 ), 0, s, a );
+            e = launch_pdl( a.u.prefetchRows ? dev::k_temporal< M, true, true, true, 128, 8, false, true > : dev::k_temporal< M, true, true, true, 128, 8 >, tgrid, dim3( 32, 4 ), 0, s, a );
             break;
         case KF_TEMPORAL_FAST_EARLY:
-            e = launch_pdl( dev::k_temporal< M, true, true, false, 128, 8, true >, dim3( grid.x, ( a.u.H + 3 ) / 4 ), dim3( 32, 4 ), 0, s, a );
+            e = launch_pdl( a.u.prefetchRows ? dev::k_temporal< M, true, true, false, 128, 8, true, true > : dev::k_temporal< M, true, true, false, 128, 8, true >, tgrid, dim3( 32, 4 ), 0, s, a );
             break;
         case KF_TEMPORAL_FAST_GP_EARLY:
-            e = launch_pdl( dev::k_temporal< M, true, true, true, 128, 8, true >, dim3( grid.x, ( a.u.H + 3 ) / 4 ), dim3( 32, 4 ), 0, s, a );
+            e = launch_pdl( a.u.prefetchRows ? dev::k_temporal< M, true, true, true, 128, 8, true, true > : dev::k_temporal< M, true, true, true, 128, 8, true >, tgrid, dim3( 32, 4 ), 0, s, a );
             break;
         case KF_ANTI_FIREFLY_FAST:
-            e = launch_pdl( dev::k_antifirefly_fast< M >, dim3( grid.x, ( a.u.H + dev::AfShared< M >::TH - 1 ) / dev::AfShared< M >::TH ), blk, 0, s, a );
+            e = launch_pdl( a.u.prefetchRows ? dev::k_antifirefly_fast< M, true > : dev::k_antifirefly_fast< M, false >, dim3( grid.x, ( a.u.H + dev::AfShared< M >::TH - 1 ) / dev::AfShared< M >::TH ), blk, 0, s, a );
             break;
         case KF_VARIANCE_EXACT_GEOM: e = launch_pdl( dev::k_variance_geo< M, false >, grid, blk, 0, s, a ); break;
         case RGDN_STAGE_ANTI_FIREFLY: dev::k_antifirefly< M ><<< grid, blk, 0, s >>>( a ); break;
@@ -4062,13 +4144,14 @@ template< int M > cudaError_t launch_atrous_pair01( const FrameArgs& a, cudaStre
 template< int M, bool HIST > cudaError_t launch_atrous_fast( const FrameArgs& a, const int iter, cudaStream_t s )
 {
     const dim3 grid( ( a.u.W + 31 ) / 32, ( a.u.H + 3 ) / 4 ), blk( 32, 4 );
+    const bool pf = a.u.prefetchRows != 0;
     switch( iter )
     {
-        case 0: return launch_pdl( dev::k_atrous< M, true, HIST, true, 128, 7, 0 >, grid, blk, 0, s, a, iter );
-        case 1: return launch_pdl( dev::k_atrous< M, true, HIST, true, 128, 7, 1 >, grid, blk, 0, s, a, iter );
-        case 2: return launch_pdl( dev::k_atrous< M, true, HIST, true, 128, 7, 2 >, grid, blk, 0, s, a, iter );
-        case 3: return launch_pdl( dev::k_atrous< M, true, HIST, true, 128, 7, 3 >, grid, blk, 0, s, a, iter );
-        case 4: return launch_pdl( dev::k_atrous< M, true, HIST, true, 128, 7, 4 >, grid, blk, 0, s, a, iter );
+        case 0: return launch_pdl( pf ? dev::k_atrous< M, true, HIST, true, 128, 7, 0, true > : dev::k_atrous< M, true, HIST, true, 128, 7, 0 >, grid, blk, 0, s, a, iter );
+        case 1: return launch_pdl( pf ? dev::k_atrous< M, true, HIST, true, 128, 7, 1, true > : dev::k_atrous< M, true, HIST, true, 128, 7, 1 >, grid, blk, 0, s, a, iter );
+        case 2: return launch_pdl( pf ? dev::k_atrous< M, true, HIST, true, 128, 7, 2, true > : dev::k_atrous< M, true, HIST, true, 128, 7, 2 >, grid, blk, 0, s, a, iter );
+        case 3: return launch_pdl( pf ? dev::k_atrous< M, true, HIST, true, 128, 7, 3, true > : dev::k_atrous< M, true, HIST, true, 128, 7, 3 >, grid, blk, 0, s, a, iter );
+        case 4: return launch_pdl( pf ? dev::k_atrous< M, true, HIST, true, 128, 7, 4, true > : dev::k_atrous< M, true, HIST, true, 128, 7, 4 >, grid, blk, 0, s, a, iter );
         default: return launch_pdl( dev::k_atrous< M, true, HIST, true, 128, 7 >, grid, blk, 0, s, a, iter );
     }
 }
