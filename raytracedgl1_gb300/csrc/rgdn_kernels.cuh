@@ -1529,8 +1529,8 @@ template< int M > __global__ void __launch_bounds__( 256 ) k_variance( const Fra
 // Anti-firefly for the default path (CmAntiFirefly.comp:120-158), the same results as
 // k_antifirefly: min / max are exact in any representation of the stored values, so 16-bit
 // storage clamps on packed half2 / bf16x2 pairs without converting, fp32 on floats, and the
-// shared-exponent storage on decoded floats. Blocks whose 5x5 footprint lies inside the image
-// skip the bounds tests. Every stored colour is non-negative and finite, so the shader's
+// shared-exponent storage on half2 pairs, which hold its values exactly. Blocks whose 5x5
+// footprint lies inside the image skip the bounds tests. Every stored colour is non-negative and finite, so the shader's
 // +-1e6 initial extrema never survive the 24 taps and the first tap seeds them.
 // ==========================================================================================
 template< int M > struct AfOps;
@@ -1585,14 +1585,38 @@ template<> struct AfOps< MODE_F32 >
     __device__ static V mx( V a, V b ) { return vmax( a, b ); }
     __device__ static void st( void* p, int i, V v ) { static_cast< float4* >( p )[ i ] = make_float4( v.x, v.y, v.z, 0.0f ); }
 };
-template<> struct AfOps< MODE_REF >
+// Every shared-exponent value m * 2^(e - 24) (m < 512, e < 32) is a binary16 value: 9 significant
+// bits, a multiple of 2^-24 (binary16's least subnormal), at most 65408. So the reference formats
+// clamp on packed half2 too, with 4 blocks per SM (three floats a texel took 3), and the block
+// decodes each texel of its tile once into shared memory (af_tile_signal) instead of once per
+// column thread and halo. The pass is bound by issue; on GB300 at 1920x1080 it went from 77.5 to
+// 53.7 us (71.9 with the packed clamp but the decode per thread).
+template<> struct AfOps< MODE_REF > : AfOps< MODE_F16 >
 {
-    using V = float3;
-    __device__ static V ld( const void* p, int i ) { return e5( static_cast< const uint32_t* >( p )[ i ] ); }
-    __device__ static V zero() { return f3( 0, 0, 0 ); }
-    __device__ static V mn( V a, V b ) { return vmin( a, b ); }
-    __device__ static V mx( V a, V b ) { return vmax( a, b ); }
-    __device__ static void st( void* p, int i, V v ) { static_cast< uint32_t* >( p )[ i ] = encode_e5( v.x, v.y, v.z ); }
+    __device__ static V decode( uint32_t p )
+    {
+        // (2^23 + m) s - 2^23 s with one rounding: m s exactly, without a conversion of m
+        const float   sc = __uint_as_float( ( ( p >> 27 ) + 103u ) << 23 ), k = -8388608.0f * sc;
+        const float   r  = __fmaf_rn( __uint_as_float( 0x4B000000u | ( p & 0x1FFu ) ), sc, k );
+        const float   g  = __fmaf_rn( __uint_as_float( 0x4B000000u | ( ( p >> 9 ) & 0x1FFu ) ), sc, k );
+        const float   b  = __fmaf_rn( __uint_as_float( 0x4B000000u | ( ( p >> 18 ) & 0x1FFu ) ), sc, k );
+        const __half2 h0 = __floats2half2_rn( r, g ), h1 = __floats2half2_rn( b, 0.0f );
+        return make_uint2( *reinterpret_cast< const uint32_t* >( &h0 ), *reinterpret_cast< const uint32_t* >( &h1 ) );
+    }
+    // encode_e5 of channels that are shared-exponent values themselves: the largest scales to an
+    // integer below 512, and the others' scaled values are short enough for an exact + 0.5
+    __device__ static uint32_t encode( V v )
+    {
+        const float r = h2f( (uint16_t)( v.x & 0xFFFFu ) ), g = h2f( (uint16_t)( v.x >> 16 ) ), b = h2f( (uint16_t)( v.y & 0xFFFFu ) );
+        const float m = fmaxf( r, fmaxf( g, b ) );
+        if( m == 0.0f ) return 0u;
+        const int      e = max( (int)( __float_as_uint( m ) >> 23 ) - 127, -16 ) + 16;
+        const float    s = exp2i( 24 - e );
+        const uint32_t ri = (uint32_t)( r * s + 0.5f ), gi = (uint32_t)( g * s + 0.5f ), bi = (uint32_t)( b * s + 0.5f );
+        return ( (uint32_t)e << 27 ) | ( bi << 18 ) | ( gi << 9 ) | ri;
+    }
+    __device__ static V    ld( const void* p, int i ) { return decode( static_cast< const uint32_t* >( p )[ i ] ); }
+    __device__ static void st( void* p, int i, V v ) { static_cast< uint32_t* >( p )[ i ] = encode( v ); }
 };
 
 template< int M, bool INTERIOR >
@@ -1654,7 +1678,10 @@ template< int M > struct AfPair
 template< int M > struct AfShared
 {
     static constexpr int RP = AfOpsRows< M >::RP, TH = 8 * RP, RW = 32 + 4;
-    AfPair< M >          v5[ TH ][ RW ];
+    // the reference formats' texels are decoded once into here: columns -2 .. 33, rows -2 .. TH + 1
+    static constexpr int TILE = M == MODE_REF ? RW * ( TH + 4 ) : 0;
+    AfPair< M >           v5[ TH ][ RW ];
+    typename AfOps< M >::V tile[ TILE ? TILE : 1 ];
 };
 static_assert( sizeof( AfShared< MODE_F32 > ) <= 48 * 1024 && sizeof( AfShared< MODE_F16 > ) <= 48 * 1024,
                "the anti-firefly tile must fit static shared memory" );
@@ -1675,7 +1702,8 @@ __device__ __forceinline__ void af_column( const Uniform& u, const void* src, co
     for( int k = 0; k < RP + 4; k++ )
     {
         const int y = r0 - 2 + k;
-        v[ k ]      = ( colIn && y >= 0 && y < u.H ) ? O::ld( src, y * u.W + x ) : O::zero();
+        if constexpr( AfShared< M >::TILE > 0 ) v[ k ] = sh.tile[ ( row0 + k ) * AfShared< M >::RW + col ];
+        else v[ k ] = ( colIn && y >= 0 && y < u.H ) ? O::ld( src, y * u.W + x ) : O::zero();
     }
 #pragma unroll
     for( int r = 0; r < RP; r++ )
@@ -1709,6 +1737,16 @@ __device__ __forceinline__ void af_tile_signal( const Uniform& u, const void* sr
     const int     tx = threadIdx.x, ty = threadIdx.y;
     V             c[ RP ];
     AfPair< M >   v4[ RP ];
+    if constexpr( AfShared< M >::TILE > 0 )
+    {
+        const int y0 = r0 - ty * RP - 2;
+        for( int k = ty * 32 + tx; k < AfShared< M >::TILE; k += 256 )
+        {
+            const int qx = bx * 32 - 2 + k % AfShared< M >::RW, qy = y0 + k / AfShared< M >::RW;
+            sh.tile[ k ] = inside( u, qx, qy ) ? O::ld( src, qy * u.W + qx ) : O::zero();
+        }
+        __syncthreads();
+    }
     af_column< M >( u, src, x, r0, sh, ty * RP, tx + 2, c, v4 );
     // the halo columns: local 0, 1 (x0 - 2, x0 - 1) and 34, 35 (x0 + 32, x0 + 33)
     if( tx < 4 )
@@ -1768,7 +1806,7 @@ template< int M > __device__ __forceinline__ void antifirefly_fast_tile( const F
     }
 }
 
-template< int M, bool PF > __global__ void __launch_bounds__( 256, ( M == MODE_F16 || M == MODE_BF16 ) ? 4 : 3 ) k_antifirefly_fast( const FrameArgs a )
+template< int M, bool PF > __global__ void __launch_bounds__( 256, M == MODE_F32 ? 3 : 4 ) k_antifirefly_fast( const FrameArgs a )
 {
     __shared__ AfShared< M > sh;
     pdl_launch_dependents();
@@ -1817,7 +1855,7 @@ template< int M > struct AfRaw;
 template<> struct AfRaw< MODE_REF >
 {
     using R = uint32_t;
-    __device__ static R      raw( float3 v ) { return encode_e5( v.x, v.y, v.z ); }
+    __device__ static R      raw( uint2 v ) { return AfOps< MODE_REF >::encode( v ); }
     __device__ static R      zero() { return 0u; }
     __device__ static float3 col( R r ) { return e5( r ); }
 };
@@ -1935,7 +1973,7 @@ template< int M, bool FAST > __device__ __forceinline__ void af_variance_tile( c
 }
 
 template< int M, bool FAST >
-__global__ void __launch_bounds__( 256, ( M == MODE_F16 || M == MODE_BF16 ) ? 4 : 3 ) k_af_variance( const FrameArgs a )
+__global__ void __launch_bounds__( 256, M == MODE_F32 ? 3 : 4 ) k_af_variance( const FrameArgs a )
 {
     __shared__ AfVarShared< M > sh;
     pdl_launch_dependents();

@@ -33,3 +33,29 @@ def test_b10g11r11_codes(mode_name, mode, omode, albedo_from_codes):
         same = (g == c) if mode == N.STORAGE_REF else (g == c) | (np.isnan(g) & np.isnan(c))
         assert same.all(), np.argwhere(~same)[:5]
         s.close()
+
+
+# one tile, cut tiles, several tiles with an odd height
+@pytest.mark.parametrize("size", [(2, 1), (32, 32), (34, 33), (98, 67)])
+@pytest.mark.parametrize("spread", [32, 3])
+def test_shared_exponent_antifirefly_any_code(size, spread):
+    """Anti-firefly in the reference formats on arbitrary codes (exponents far apart and close, unnormalised
+    mantissas, zeros): the packed kernel equals the one that clamps decoded floats, bit for bit."""
+    W, H = size
+    rng = np.random.default_rng(W * 100 + spread)
+    _, p = Scene(W, H, seed=3).generate(0)
+    with Context(0) as ctx:
+        a, b = Stream(ctx, W, H, N.STORAGE_REF), Stream(ctx, W, H, N.STORAGE_REF)
+        for name in ("DIFF_TEMPORARY", "SPEC_ACCUM_COLOR", "INDIR_ACCUM"):
+            code = rng.integers(0, 2 ** 27, (H, W), dtype=np.uint64) | (rng.integers(0, spread, (H, W), dtype=np.uint64) << 27)
+            code[rng.random((H, W)) < 0.1] = 0
+            for s in (a, b):
+                s.upload(name, 0, code.astype(np.uint32))
+        q = p.copy()
+        q.flags |= N.FLAG_STAGE_DEFAULT
+        a.stage(N.STAGE_ANTI_FIREFLY, 0, 0, p)
+        b.stage(N.STAGE_ANTI_FIREFLY, 0, 0, q)
+        for name in ("DIFF_ACCUM_COLOR", "SPEC_PING_COLOR", "INDIR_PING"):
+            assert np.array_equal(a.download(name, 0), b.download(name, 0)), name
+        a.close()
+        b.close()
