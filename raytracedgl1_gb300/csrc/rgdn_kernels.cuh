@@ -938,8 +938,12 @@ constexpr bool kTemporalEarlySurfPos = false;
 // 4 % faster; with the geometry record persisting in L2 and the other later changes the pass ran
 // 98.8 us without the prefetch against 102.4 with it, A/B/A/B on GB300)
 constexpr bool kTemporalL2Prefetch = false;
-// the temporal pass reads this frame's unfiltered colours and view ray before its taps
-constexpr bool kTemporalEarlyInputs = true;
+// The temporal pass reads this frame's unfiltered colours and view ray after its taps where they are
+// in L2 by then and would only hold registers across the tap loop (the default path: 91.2 us with them
+// first and 89.1 after at 1920x1080 fp16, 339 and 331 at 3840x2160 bf16, 55.4 and 53.6 at 1366x767), and
+// before them in the IEEE form, which has registers to spare (121.8 first, 127.4 after, at 1280x720
+// fp32), and in the reference formats (97.9 and 98.3).
+template< int M, bool FAST > constexpr bool kTemporalEarlyInputs = !FAST || M == MODE_REF;
 template< int M, bool FAST, bool GEOM, bool GEOMPREV, bool EARLY = false >
 __device__ __forceinline__ void temporal_tile( const FrameArgs& a, int bx, int by, const float* u8 )
 {
@@ -962,7 +966,7 @@ __device__ __forceinline__ void temporal_tile( const FrameArgs& a, int bx, int b
         const ushort4 rv   = a.viewDir[ i ];
         rayInfo            = make_float4( h2f( rv.x ), h2f( rv.y ), h2f( rv.z ), h2f( rv.w ) );
     };
-    if( kTemporalEarlyInputs ) ldInputs();
+    if( kTemporalEarlyInputs< M, FAST > ) ldInputs();
     const Area     chArea          = cb_area( u, px );
     const ushort4  mo              = a.motion[ i ];
     const float    motionZ         = h2f( mo.z );
@@ -1114,7 +1118,7 @@ __device__ __forceinline__ void temporal_tile( const FrameArgs& a, int bx, int b
         }
     }
 
-    if( !kTemporalEarlyInputs ) ldInputs();
+    if( !kTemporalEarlyInputs< M, FAST > ) ldInputs();
     const float  l          = X::lum( unfilteredDiff );
     const float2 moments    = make_float2( l, l * l );
     const bool   hasHistory = weightSum > 0.0001f;
