@@ -2431,14 +2431,19 @@ __global__ void __launch_bounds__( NT, MINB ) k_atrous( const FrameArgs a, const
     if constexpr( PF )
     {
         const AtrousIO io = atrous_io< M >( a, iter );
-        prefetch_ahead< 6, NT / 32 >( a.u, t, 1 << iter, [ & ]( int k, const void*& p, int& e ) {
+        prefetch_ahead< HIST ? 9 : 6, NT / 32 >( a.u, t, 1 << iter, [ & ]( int k, const void*& p, int& e ) {
             using B = TexelBytes< M >;
             if( k == 0 ) p = a.geom, e = 16;
             else if( k == 1 ) p = io.diffSrc, e = B::cv;
             else if( k == 2 ) p = io.specSrc, e = B::colour;
             else if( k == 3 ) p = io.indirSrc, e = B::colour;
             else if( k == 4 ) p = a.histLen, e = B::cv;
-            else if( Sto< M >::varPlane ) p = io.varSrc, e = 4;
+            else if( k == 5 ) p = Sto< M >::varPlane ? io.varSrc : nullptr, e = 4;
+            // the composition's inputs (the albedo's, in the regular layout, measured slower: two blocks
+            // share its rows)
+            else if( k == 6 ) p = a.throughput, e = 8;
+            else if( k == 7 ) p = a.isSky, e = 1;
+            else p = a.mr, e = 2;
         } );
     }
     atrous_tile< M, FAST, HIST, GEOMIN >( a, iter, blockIdx.x, blockIdx.y, u8, hist );
