@@ -3481,7 +3481,7 @@ template< int M, bool FAST > __global__ void __launch_bounds__( 256 ) k_prepare_
     pdl_wait();
     // The pixel's texels, in flight while one thread evaluates the exposure below: asked for after
     // the barrier, each block waited for the average's load, the log and exponential, and only then
-    // for memory (39.1 us instead of 44.2 at 2560x1440 FP16).
+    // for memory (tonemap and bloom of 2560x1440 FP16: 159.4 us, 164.6 before).
     const int  i   = y * f.W + x;
     const bool in  = x < f.W && y < f.H;
     // getCheckerboardPix (ShaderCommonGLSLFunc.h:321-329)
@@ -3568,9 +3568,12 @@ template< int M, bool FAST > __global__ void __launch_bounds__( 256 ) k_prepare_
 // images in PRE_FINAL's format. textureLod with the framebuffers' bilinear clamp-to-edge
 // sampler is evaluated in FP32 (texel centres at +0.5, weights from the fractional position).
 // ==========================================================================================
-// One bloom texel: (r, g) as a pair for the packed FP32x2 operations, b alone. Each packed
-// lane rounds as the scalar operation does (no contraction), so results equal a scalar
-// evaluation bit for bit.
+// One bloom texel: (r, g) as a pair for the packed FP32x2 operations, b alone. Each packed lane
+// rounds as the scalar operation does. The passes are bound by issue (64 to 67 % of the slots at
+// 2560x1440), so outside the reference formats the weighted sums are fused multiply-adds: one
+// operation and one rounding less for each tap (bloom of 2560x1440 FP16: 120.7 us, 128.5 before;
+// the quad upsample holds 76 registers, 90 before). The reference formats are packed integers
+// whose bytes follow the uncontracted sums.
 struct P3
 {
     float2 rg;
@@ -3579,11 +3582,20 @@ struct P3
 __device__ __forceinline__ float3 f3of( P3 p ) { return f3( p.rg.x, p.rg.y, p.b ); }
 __device__ __forceinline__ P3     padd( P3 a, P3 b ) { return { __fadd2_rn( a.rg, b.rg ), a.b + b.b }; }
 __device__ __forceinline__ P3     pmul( P3 a, float s ) { return { __fmul2_rn( a.rg, make_float2( s, s ) ), a.b * s }; }
-// gmix per channel: x (1 - a) + y a
-__device__ __forceinline__ P3 pmix( P3 x, P3 y, float a )
+// gmix per channel: x (1 - a) + y a; outside the reference formats the sum is a fused multiply-add
+// (one operation and one rounding less per channel)
+template< int M > __device__ __forceinline__ P3 pmix( P3 x, P3 y, float a )
 {
     const float w = 1.0f - a;
+    if constexpr( M != MODE_REF )
+        return { __ffma2_rn( y.rg, make_float2( a, a ), __fmul2_rn( x.rg, make_float2( w, w ) ) ), __fmaf_rn( y.b, a, x.b * w ) };
     return { __fadd2_rn( __fmul2_rn( x.rg, make_float2( w, w ) ), __fmul2_rn( y.rg, make_float2( a, a ) ) ), x.b * w + y.b * a };
+}
+// r + s c
+template< int M > __device__ __forceinline__ P3 pmadd( P3 r, P3 c, float s )
+{
+    if constexpr( M != MODE_REF ) return { __ffma2_rn( c.rg, make_float2( s, s ), r.rg ), __fmaf_rn( c.b, s, r.b ) };
+    return padd( r, pmul( c, s ) );
 }
 __device__ __forceinline__ float plum( P3 c ) { return 0.2125f * c.rg.x + 0.7154f * c.rg.y + 0.0721f * c.b; }
 
@@ -3612,7 +3624,7 @@ template< int M > __device__ __forceinline__ P3 bl_sample( const void* img, int 
 {
     const P3 t00 = bloom_ld< M >( img, (size_t)( ay.i0 * w + ax.i0 ) ), t10 = bloom_ld< M >( img, (size_t)( ay.i0 * w + ax.i1 ) );
     const P3 t01 = bloom_ld< M >( img, (size_t)( ay.i1 * w + ax.i0 ) ), t11 = bloom_ld< M >( img, (size_t)( ay.i1 * w + ax.i1 ) );
-    return pmix( pmix( t00, t10, ax.f ), pmix( t01, t11, ax.f ), ay.f );
+    return pmix< M >( pmix< M >( t00, t10, ax.f ), pmix< M >( t01, t11, ax.f ), ay.f );
 }
 
 // One texel of downsample step k (CmBloomDownsample.comp:15-136): src is BLOOM_INPUT (k = 0)
@@ -3658,21 +3670,21 @@ __device__ __forceinline__ void bloom_down_texel( const void* src, int sw, int s
             for( int c = 0; c < 6; c++ ) t[ c ] = bloom_ld< M >( src, (size_t)( row * sw + col[ c ] ) );
 #pragma unroll
             for( int j = 0; j < 5; j++ )
-                if( ( j & 1 ) == 0 || ( r >= 1 && r <= 4 ) ) hc[ j ] = pmix( t[ j ], t[ j + 1 ], ax[ j ].f );
+                if( ( j & 1 ) == 0 || ( r >= 1 && r <= 4 ) ) hc[ j ] = pmix< M >( t[ j ], t[ j + 1 ], ax[ j ].f );
             if( r > 0 )
             {
                 const int   yj = r - 1;
                 const float b  = ay[ yj ].f;
                 if( ( yj & 1 ) == 0 )
                 {
-                    const P3 ta = pmix( hp[ 0 ], hc[ 0 ], b ), tb = pmix( hp[ 2 ], hc[ 2 ], b ), tc = pmix( hp[ 4 ], hc[ 4 ], b );
+                    const P3 ta = pmix< M >( hp[ 0 ], hc[ 0 ], b ), tb = pmix< M >( hp[ 2 ], hc[ 2 ], b ), tc = pmix< M >( hp[ 4 ], hc[ 4 ], b );
                     if( yj == 0 ) s1 = padd( ta, tb ), s2 = padd( tb, tc );
                     else if( yj == 2 ) s1 = padd( padd( s1, ta ), tb ), s2 = padd( padd( s2, tb ), tc ), s3 = padd( ta, tb ), s4 = padd( tb, tc );
                     else s3 = padd( padd( s3, ta ), tb ), s4 = padd( padd( s4, tb ), tc );
                 }
                 else
                 {
-                    const P3 ta = pmix( hp[ 1 ], hc[ 1 ], b ), tb = pmix( hp[ 3 ], hc[ 3 ], b );
+                    const P3 ta = pmix< M >( hp[ 1 ], hc[ 1 ], b ), tb = pmix< M >( hp[ 3 ], hc[ 3 ], b );
                     s0 = yj == 1 ? padd( ta, tb ) : padd( padd( s0, ta ), tb );
                 }
             }
@@ -3698,9 +3710,9 @@ __device__ __forceinline__ void bloom_down_texel( const void* src, int sw, int s
     {
         // partial Karis average: each box weighted by 1 / (1 + luminance)
         auto kw = []( P3 bx ) { return 1.0f / ( 1.0f + plum( bx ) ); };
-        r       = padd( padd( padd( padd( pmul( b0, 0.5f * kw( b0 ) ), pmul( b1, 0.125f * kw( b1 ) ) ), pmul( b2, 0.125f * kw( b2 ) ) ),
-                              pmul( b3, 0.125f * kw( b3 ) ) ),
-                        pmul( b4, 0.125f * kw( b4 ) ) );
+        r       = pmadd< M >( pmadd< M >( pmadd< M >( pmadd< M >( pmul( b0, 0.5f * kw( b0 ) ), b1, 0.125f * kw( b1 ) ), b2, 0.125f * kw( b2 ) ), b3,
+                                          0.125f * kw( b3 ) ),
+                              b4, 0.125f * kw( b4 ) );
     }
     else r = padd( padd( padd( padd( pmul( b0, 0.5f ), pmul( b1, 0.125f ) ), pmul( b2, 0.125f ) ), pmul( b3, 0.125f ) ), pmul( b4, 0.125f ) );
     Sto< M >::stpre( dst, (size_t)( y * dw + x ), f3of( r ) );
@@ -3740,10 +3752,10 @@ __device__ __forceinline__ void bloom_up_texel( const void* src, int sw, int sh,
 #pragma unroll
             for( int c = 0; c < 4; c++ ) t[ c ] = bloom_ld< M >( src, (size_t)( row * sw + col[ c ] ) );
 #pragma unroll
-            for( int j = 0; j < 3; j++ ) hc[ j ] = pmix( t[ j ], t[ j + 1 ], ax[ j ].f );
+            for( int j = 0; j < 3; j++ ) hc[ j ] = pmix< M >( t[ j ], t[ j + 1 ], ax[ j ].f );
             if( rr > 0 )
 #pragma unroll
-                for( int j = 0; j < 3; j++ ) r = padd( r, pmul( pmix( hp[ j ], hc[ j ], ay[ rr - 1 ].f ), wt( rr - 1, j ) ) );
+                for( int j = 0; j < 3; j++ ) r = pmadd< M >( r, pmix< M >( hp[ j ], hc[ j ], ay[ rr - 1 ].f ), wt( rr - 1, j ) );
 #pragma unroll
             for( int j = 0; j < 3; j++ ) hp[ j ] = hc[ j ];
         }
@@ -3753,7 +3765,7 @@ __device__ __forceinline__ void bloom_up_texel( const void* src, int sw, int sh,
 #pragma unroll
         for( int q = 0; q < 3; q++ )
 #pragma unroll
-            for( int j = 0; j < 3; j++ ) r = padd( r, pmul( bl_sample< M >( src, sw, ax[ j ], ay[ q ] ), wt( q, j ) ) );
+            for( int j = 0; j < 3; j++ ) r = pmadd< M >( r, bl_sample< M >( src, sw, ax[ j ], ay[ q ] ), wt( q, j ) );
     }
     if( k > 0 ) r = padd( r, bloom_ld< M >( dst, (size_t)( y * dw + x ) ) );
     Sto< M >::stpre( dst, (size_t)( y * dw + x ), f3of( r ) );
@@ -3818,7 +3830,7 @@ __device__ __forceinline__ bool bloom_up_quad( const void* src, int sw, int sh, 
 #pragma unroll
         for( int xi = 0; xi < 2; xi++ )
 #pragma unroll
-            for( int j = 0; j < 3; j++ ) hc[ xi ][ j ] = pmix( t[ j ], t[ j + 1 ], ax[ xi ][ j ].f );
+            for( int j = 0; j < 3; j++ ) hc[ xi ][ j ] = pmix< M >( t[ j ], t[ j + 1 ], ax[ xi ][ j ].f );
         if( rr > 0 )
 #pragma unroll
             for( int yi = 0; yi < 2; yi++ )
@@ -3826,7 +3838,7 @@ __device__ __forceinline__ bool bloom_up_quad( const void* src, int sw, int sh, 
                 for( int xi = 0; xi < 2; xi++ )
 #pragma unroll
                     for( int j = 0; j < 3; j++ )
-                        r[ yi ][ xi ] = padd( r[ yi ][ xi ], pmul( pmix( hp[ xi ][ j ], hc[ xi ][ j ], ay[ yi ][ rr - 1 ].f ), wt( rr - 1, j ) ) );
+                        r[ yi ][ xi ] = pmadd< M >( r[ yi ][ xi ], pmix< M >( hp[ xi ][ j ], hc[ xi ][ j ], ay[ yi ][ rr - 1 ].f ), wt( rr - 1, j ) );
 #pragma unroll
         for( int xi = 0; xi < 2; xi++ )
 #pragma unroll
