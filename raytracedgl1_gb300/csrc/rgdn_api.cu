@@ -1143,6 +1143,7 @@ rgdn_status rgdn_process_scattering( rgdn_stream* s, uint32_t frameIndex, const 
     a.enableType       = p->volumeEnableType;
     a.frameId          = p->frameId;
     a.flags            = p->flags;
+    a.unfused          = s->storage == RGDN_STORAGE_REF;
     a.irw              = 1.0f / a.u.rw;
     a.irh              = 1.0f / a.u.rh;
     a.iRange           = 1.0f / ( a.volFar - a.volNear );

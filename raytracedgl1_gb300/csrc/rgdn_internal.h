@@ -211,6 +211,7 @@ struct ScatterArgs
     uint32_t       enableType;
     uint32_t       frameId;
     uint32_t       flags;             // RGDN_VOLUME_EXACT_MATH
+    bool           unfused;           // the stream's composition packs integers: no fused multiply-adds
 };
 cudaError_t launch_process_scattering( const ScatterArgs& a, cudaStream_t s );
 cudaError_t launch_final_ref( const FinalArgs& f, cudaStream_t s );

@@ -4124,7 +4124,11 @@ __device__ __forceinline__ float3 volume_dithered_pos_fast( const ScatterArgs& a
 // Nothing before the wait reads the volume, so the reprojection overlaps the volume pass, which
 // leaves most of the chip idle: everything else it reads was complete before that pass let this
 // grid start (k_volume_process).
-template< bool FAST >
+//
+// FMA: the fused form of the FAST arithmetic. Streams in the reference formats keep the unfused one:
+// the composition packs what it reads here into 11- and 10-bit integers, and the fused form's last bit
+// moved 0.03 % of those.
+template< bool FAST, bool FMA >
 __device__ __forceinline__ float4 scatter_pixel( const ScatterArgs& a, int cx, int cy, const float* inv255, float& histOut )
 {
     const int      W     = a.u.W;
@@ -4166,7 +4170,7 @@ __device__ __forceinline__ float4 scatter_pixel( const ScatterArgs& a, int cx, i
             {
                 const float  w = bw[ yy ][ xx ];
                 const float4 v = h4f( sv );
-                if constexpr( FAST )
+                if constexpr( FMA )
                 {
                     acc  = make_float4( __fmaf_rn( w, v.x, acc.x ), __fmaf_rn( w, v.y, acc.y ), __fmaf_rn( w, v.z, acc.z ), __fmaf_rn( w, v.w, acc.w ) );
                     hist = __fmaf_rn( w, h2f( hv ), hist );
@@ -4194,7 +4198,7 @@ __device__ __forceinline__ float4 scatter_pixel( const ScatterArgs& a, int cx, i
     hist           = gclamp( hist + 1.0f, 1.0f, fmaxf( 1.0f, a.maxHistoryLength ) );
     const int2 reg = regular_from_cb( a.u, cx, cy );
     histOut        = hist;
-    if constexpr( FAST )
+    if constexpr( FMA )
     {
         float4 now;
         if( a.enableType == RGDN_VOLUME_ENABLE_VOLUMETRIC )
@@ -4213,7 +4217,7 @@ __device__ __forceinline__ float4 scatter_pixel( const ScatterArgs& a, int cx, i
                             __fmaf_rn( f, now.w - acc.w, acc.w ) );
     }
     pdl_wait();
-    return vmix4( acc, finalize_scattering< FAST >( a, reg.x, reg.y, depth, inv255 ), 1.0f / hist );
+    return vmix4( acc, finalize_scattering< FAST >( a, reg.x, reg.y, depth, inv255 ), FAST ? rcp_approx( hist ) : 1.0f / hist );
 }
 
 // One thread per checkerboard pixel. (One thread per pair (cx, cx + W/2), whose regular pixels
@@ -4223,10 +4227,10 @@ __device__ __forceinline__ float4 scatter_pixel( const ScatterArgs& a, int cx, i
 // 75.1 to 54 us (978 to 720 instructions a pixel: fused multiply-adds and packed lerps, 32-bit
 // offsets, no table of byte / 255 to fill) and the two passes together from 86.2 to 67.3, the volume
 // pass being overlapped. 6 blocks per SM: 5 took 69.8 us, 7 (36 registers) 75.6.
-template< int M, bool FAST > __global__ void __launch_bounds__( 256, 6 ) k_scatter_accum( const ScatterArgs a )
+template< int M, bool FAST, bool FMA > __global__ void __launch_bounds__( 256, 6 ) k_scatter_accum( const ScatterArgs a )
 {
-    __shared__ float inv255[ FAST ? 1 : 256 ];
-    if( !FAST )
+    __shared__ float inv255[ FMA ? 1 : 256 ];
+    if( !FMA )
     {
         for( int t = threadIdx.y * blockDim.x + threadIdx.x; t < 256; t += blockDim.x * blockDim.y ) inv255[ t ] = u8_value( t );
         __syncthreads();
@@ -4235,7 +4239,7 @@ template< int M, bool FAST > __global__ void __launch_bounds__( 256, 6 ) k_scatt
     pdl_launch_dependents();
     if( cx >= a.u.W || cy >= a.u.H ) return;
     float        hist;
-    const float4 acc = scatter_pixel< FAST >( a, cx, cy, inv255, hist );
+    const float4 acc = scatter_pixel< FAST, FMA >( a, cx, cy, inv255, hist );
     const int2   reg = regular_from_cb( a.u, cx, cy );
     const int    ri  = reg.y * a.u.W + reg.x;
     a.scatterOut[ ri ] = f4h( acc );
@@ -4329,8 +4333,9 @@ template< int M > cudaError_t launch_scatter_t( const ScatterArgs& a, cudaStream
                                 a.nz * dev::kVolumeBlock * sizeof( ushort4 ), s, a.volume, a.nx, a.ny, a.nz );
     const dim3 g( ( a.u.W + 31 ) / 32, ( a.u.H + 7 ) / 8 ), b( 32, 8 );
     if( e == cudaSuccess )
-        e = ( a.flags & RGDN_VOLUME_EXACT_MATH ) ? launch_pdl( dev::k_scatter_accum< M, false >, g, b, 0, s, a )
-                                                  : launch_pdl( dev::k_scatter_accum< M, true >, g, b, 0, s, a );
+        e = ( a.flags & RGDN_VOLUME_EXACT_MATH ) ? launch_pdl( dev::k_scatter_accum< M, false, false >, g, b, 0, s, a )
+            : a.unfused                          ? launch_pdl( dev::k_scatter_accum< M, true, false >, g, b, 0, s, a )
+                                                 : launch_pdl( dev::k_scatter_accum< M, true, true >, g, b, 0, s, a );
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 

@@ -1,0 +1,40 @@
+"""ProcessScattering of a stream in the reference formats takes the unfused form of the default
+arithmetic: the same bounds against the oracle as the fused form of the other storage modes."""
+import numpy as np
+import pytest
+
+import oracle
+from raytracedgl1_gb300 import _native as N
+from raytracedgl1_gb300.denoiser import Context, Stream, Volumetric
+from raytracedgl1_gb300.scene import Scene
+from tests import _formats as F
+from tests.test_gpu_parity import TOL, _volumetric_params, upload_frame
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("vmode", [N.VOLUME_ENABLE_SIMPLE, N.VOLUME_ENABLE_VOLUMETRIC])
+@pytest.mark.parametrize("size", [(64, 36), (50, 23)])
+def test_scattering_of_a_reference_stream(vmode, size):
+    W, H = size
+    rng = np.random.default_rng(W * 37 + H + vmode)
+    s = Stream(Context(), W, H, N.STORAGE_REF)
+    o = oracle.OracleStream(W, H, oracle.MODE_F32)
+    nx, ny, nz = N.VOLUME_SIZE
+    vol = np.concatenate([rng.uniform(0, 0.5, (ny * nz, nx, 3)), rng.uniform(0, 0.1, (ny * nz, nx, 1))], axis=2)
+    upload_frame(s, o, {"SCATTER_VOLUME": vol.astype(np.float16).view(np.uint16)}, 0)
+    prev = np.concatenate([rng.uniform(0, 1, (H, W, 3)), rng.uniform(0.2, 1, (H, W, 1))], axis=2)
+    upload_frame(s, o, {"SCATTERING": prev.astype(np.float16).view(np.uint16),
+                        "SCATTERING_HISTORY": rng.uniform(1, 5, (H, W)).astype(np.float16).view(np.uint16)}, 1)
+    bufs, _ = Scene(W, H, seed=W + vmode).generate(0)
+    upload_frame(s, o, {k: bufs[k] for k in ("NORMAL", "DEPTH_WORLD", "MOTION")}, 0)
+    upload_frame(s, o, {"DEPTH_NDC": rng.uniform(0.1, 0.9, (H, W)).astype(np.float32)}, 0)
+    p = _volumetric_params(vmode, 100)
+    Volumetric(s).ProcessScattering(0, p)
+    o.process_scattering(0, p)
+    for name in ("SCATTERING", "SCATTERING_HISTORY"):
+        img = s.image(name, 0)
+        err = F.texel_rel_err(F.decode(s.download(name, 0), img.format), F.decode(o.plane(name, 0), img.format), atol=1e-6)
+        assert err.max() <= TOL[img.format], f"{name}: max rel err {err.max():.3e}"
+        assert np.mean(err > 0) <= 0.02, f"{name}: {np.mean(err > 0):.2%} of texels differ"
+    s.close()
