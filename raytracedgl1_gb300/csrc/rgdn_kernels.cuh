@@ -877,7 +877,11 @@ __device__ __forceinline__ void gradient_atrous_tile( const FrameArgs& a, int it
 // The first kernel of a frame lets its dependents launch only after its own wait: every kernel
 // enqueued before the frame has then completed, so the temporal pass that follows the gradient
 // chain may read the frame's inputs and history before its own wait (k_temporal, EARLY).
-template< int M > __global__ void __launch_bounds__( 256, 6 ) k_gradient_samples( const FrameArgs a, uint32_t* dst )
+// 4 blocks per SM: at 6 (40 registers) the kernel spilled 92 B, which small frames, with one block on
+// an SM, waited for: 320x180 FP16 49.2 us per frame against 48.5 at 4, 640x360 FP32 93.8 against 93.0,
+// 4K BF16 1648.6 against 1646.8; 1080p, one full wave at 6, measured the same (432.4). 5 blocks:
+// 1080p 432.7, 1366x767 223.6 against 223.0.
+template< int M > __global__ void __launch_bounds__( 256, 4 ) k_gradient_samples( const FrameArgs a, uint32_t* dst )
 {
     __shared__ float u8[ 256 ];
     fill_u8( u8, threadIdx.y * blockDim.x + threadIdx.x );
