@@ -3791,7 +3791,9 @@ __device__ __forceinline__ void bloom_up_texel( const void* src, int sw, int sh,
 }
 
 // MINB 4 for the large steps (more warps in flight at 64 registers), 1 for the small coarse
-// steps, whose single wave is bound by one texel's chain of dependent loads
+// steps, whose single wave is bound by one texel's chain of dependent loads. FP32's texels hold
+// twice the registers: 3 (80 registers), tonemap and bloom of 1280x720 75.6 us against 79.1 at 4;
+// at 2 (128) it spills more. FP16 measured the other way (2560x1440 152.4 at 3, 151.5 at 4).
 template< int M, int MINB >
 __global__ void __launch_bounds__( 256, MINB ) k_bloom_down( const void* src, int sw, int sh, void* dst, int dw, int dh, int k, float4 st )
 {
@@ -4313,7 +4315,7 @@ template< int M > cudaError_t launch_bloom_t( const BloomArgs& b, cudaStream_t s
                             (float)( 1 << k ) / (float)b.H );
     };
     for( int k = 0; k < 8 && e == cudaSuccess; k++ )
-        e = launch_pdl( large( k + 1 ) ? dev::k_bloom_down< M, 4 > : dev::k_bloom_down< M, 1 >, grid( b.w[ k + 1 ], b.h[ k + 1 ] ), blk, 0, s,
+        e = launch_pdl( large( k + 1 ) ? dev::k_bloom_down< M, M == MODE_F32 ? 3 : 4 > : dev::k_bloom_down< M, 1 >, grid( b.w[ k + 1 ], b.h[ k + 1 ] ), blk, 0, s,
                         (const void*)b.planes[ k ], b.w[ k ], b.h[ k ], b.planes[ k + 1 ], b.w[ k + 1 ], b.h[ k + 1 ], k, st( k ) );
     for( int k = 7; k >= 0 && e == cudaSuccess; k-- )
     {
