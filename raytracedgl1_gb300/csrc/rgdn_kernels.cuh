@@ -3996,7 +3996,9 @@ __device__ __forceinline__ float4 volume_trilinear( const ushort4* vol, int nx, 
     return vmix4( vmix4( c00, c10, fy ), vmix4( c01, c11, fy ), fz );
 }
 
-// The same with x + f (y - x) in packed FP32 pairs and 32-bit offsets (continuous in every term)
+// The same in packed FP32 pairs with 32-bit offsets, y f + x (1 - f) with the second product's
+// rounding only. Not x + f (y - x): beside each other two cells that overflowed binary16 must give
+// Inf, and their difference is NaN.
 __device__ __forceinline__ float4 volume_trilinear_fast( const ushort4* vol, float3 sp )
 {
     constexpr int NX = RGDN_VOLUME_SIZE_X, NY = RGDN_VOLUME_SIZE_Y, NZ = RGDN_VOLUME_SIZE_Z;
@@ -4022,10 +4024,9 @@ __device__ __forceinline__ float4 volume_trilinear_fast( const ushort4* vol, flo
         return P4{ __half22float2( __halves2half2( __ushort_as_half( h.x ), __ushort_as_half( h.y ) ) ),
                    __half22float2( __halves2half2( __ushort_as_half( h.z ), __ushort_as_half( h.w ) ) ) };
     };
-    auto lerp1 = []( float2 x, float2 y, float2 f ) { return __ffma2_rn( f, __fadd2_rn( y, make_float2( -x.x, -x.y ) ), x ); };
-    auto lerp  = [ & ]( const P4& x, const P4& y, float f ) {
-        const float2 ff = make_float2( f, f );
-        return P4{ lerp1( x.a, y.a, ff ), lerp1( x.b, y.b, ff ) };
+    auto lerp = []( const P4& x, const P4& y, float f ) {
+        const float2 ff = make_float2( f, f ), ww = make_float2( 1.0f - f, 1.0f - f );
+        return P4{ __ffma2_rn( y.a, ff, __fmul2_rn( x.a, ww ) ), __ffma2_rn( y.b, ff, __fmul2_rn( x.b, ww ) ) };
     };
     const int r00 = ( z0 * NY + y0 ) * NX, r10 = ( z0 * NY + y1 ) * NX, r01 = ( z1 * NY + y0 ) * NX, r11 = ( z1 * NY + y1 ) * NX;
     const P4  t0 = ld( r00, x0 ), t1 = ld( r00, x1 ), t2 = ld( r10, x0 ), t3 = ld( r10, x1 );
@@ -4218,9 +4219,10 @@ __device__ __forceinline__ float4 scatter_pixel( const ScatterArgs& a, int cx, i
             pdl_wait();
             now = finalize_scattering< true >( a, reg.x, reg.y, depth, inv255 );
         }
-        const float f = rcp_approx( hist );
-        return make_float4( __fmaf_rn( f, now.x - acc.x, acc.x ), __fmaf_rn( f, now.y - acc.y, acc.y ), __fmaf_rn( f, now.z - acc.z, acc.z ),
-                            __fmaf_rn( f, now.w - acc.w, acc.w ) );
+        // two products, as the lerps above: a history of 1 (a reset) gives `now` whatever acc was,
+        // and an infinite acc stays infinite
+        const float f = rcp_approx( hist ), w = 1.0f - f;
+        return make_float4( __fmaf_rn( now.x, f, acc.x * w ), __fmaf_rn( now.y, f, acc.y * w ), __fmaf_rn( now.z, f, acc.z * w ), __fmaf_rn( now.w, f, acc.w * w ) );
     }
     pdl_wait();
     return vmix4( acc, finalize_scattering< FAST >( a, reg.x, reg.y, depth, inv255 ), FAST ? rcp_approx( hist ) : 1.0f / hist );
