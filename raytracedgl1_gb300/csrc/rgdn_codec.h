@@ -135,6 +135,18 @@ RGDN_HD uint32_t f32_to_unorm8( float f )
     return (uint32_t)roundf( c * 255.0f );
 }
 RGDN_HD float unorm8_to_f32( uint32_t u ) { return (float)u / 255.0f; }
+// The same for a code u already in FP32, without a division or a table: u / 255 is u hi + u lo, hi the
+// binary32 nearest to 1/255 and lo the nearest to what hi leaves of it. The fused sum rounds once and
+// gives the quotient's binary32 for each of the 256 codes; u hi alone differs from it in 126.
+RGDN_HD float unorm8_product( float u )
+{
+    constexpr float hi = 1.0f / 255.0f, lo = (float)( 1.0 / 255.0 - (double)hi );
+#if defined( __CUDA_ARCH__ )
+    return __fmaf_rn( u, hi, u * lo );
+#else
+    return fmaf( u, hi, u * lo );
+#endif
+}
 
 // ---------------------------------------------------------------- E5B9G9R9 (Utils.h:162-207)
 RGDN_HD uint32_t encode_e5( float r, float g, float b )

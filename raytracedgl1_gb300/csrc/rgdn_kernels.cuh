@@ -4109,8 +4109,7 @@ __device__ __forceinline__ float3 volume_dithered_pos_fast( const ScatterArgs& a
     const float  iw = rcp_approx( p.z );
     const float3 w  = f3( p.x * iw, p.y * iw, __fmaf_rn( m[ 2 ], nx, __fmaf_rn( m[ 6 ], ny, __fmaf_rn( m[ 10 ], nz, m[ 14 ] ) ) ) * iw );
     const uint32_t rnd = wellons_lowbias32( random_seed( rx, ry, a.frameId ) );
-    // byte / 255 as a product with the reciprocal: an ulp of a dither
-    auto           unorm = [ & ]( int byte ) { return ( __uint_as_float( __byte_perm( rnd, 0x4B000000u, 0x7440 + byte ) ) - 8388608.0f ) * ( 1.0f / 255.0f ); };
+    auto           unorm = [ & ]( int byte ) { return unorm8_product( __uint_as_float( __byte_perm( rnd, 0x4B000000u, 0x7440 + byte ) ) - 8388608.0f ); };
     const float    r0 = unorm( 0 ), r1 = unorm( 1 ), r2 = unorm( 2 );
     const float    u1 = r0 * 0.99f, rr = sqrt_approx( u1 ), hz = sqrt_approx( 1.0f - u1 );
     float          sphi, cphi;

@@ -3,6 +3,7 @@ the codecs implement: IEEE-754 binary16 (numpy's float16 as the independent refe
 bfloat16 round-to-nearest-even, EXT_texture_shared_exponent (E5B9G9R9), the 11/10-bit
 unsigned floats of B10G11R11, and the spherical normal code of Utils.h:105-140."""
 import math
+import os
 
 import numpy as np
 import pytest
@@ -135,3 +136,16 @@ def test_product_bin_table_matches_oracle():
         vals = np.arange(65536, dtype=np.uint32).astype(np.uint16).view(np.float16).astype(np.float32)
         ref = np.array([oracle.color_bin(float(v), lo, hi) for v in vals], dtype=np.uint8)
         assert np.array_equal(t, ref)
+
+
+def test_unorm8_product_is_the_quotient(tmp_path):
+    """The kernels' division-free u / 255 (csrc/rgdn_codec.h, the same two operations on the host): the
+    IEEE binary32 quotient for every code. (The product with 1/255 alone misses it in 126.)"""
+    import subprocess
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "raytracedgl1_gb300", "csrc")
+    src, exe = tmp_path / "u.cpp", tmp_path / "u"
+    src.write_text('#include "rgdn_codec.h"\n#include <stdio.h>\n'
+                   'int main() { for( int k = 0; k < 256; k++ ) printf( "%08x\\n", rgdn::f2u( rgdn::unorm8_product( (float)k ) ) ); }\n')
+    subprocess.run(["g++", "-std=c++17", "-O2", "-I", csrc, str(src), "-o", str(exe)], check=True)
+    got = [int(v, 16) for v in subprocess.run([str(exe)], check=True, capture_output=True, text=True).stdout.split()]
+    assert got == (np.arange(256, dtype=np.float32) / np.float32(255.0)).view(np.uint32).tolist()
