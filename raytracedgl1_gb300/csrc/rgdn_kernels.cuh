@@ -947,12 +947,6 @@ __device__ __forceinline__ float parallax( const Uniform& u, float3 pos, float3 
 // at the taps.
 // the temporal pass reads each in-area tap's history together with its geometry
 constexpr bool kTemporalEarlyHistory = true;
-// the temporal pass reads the surface positions before the taps rather than where they are used
-constexpr bool kTemporalEarlySurfPos = false;
-// the temporal pass prefetches the history rows under its bilinear footprint into L2 (once
-// 4 % faster; with the geometry record persisting in L2 and the other later changes the pass ran
-// 98.8 us without the prefetch against 102.4 with it, A/B/A/B on GB300)
-constexpr bool kTemporalL2Prefetch = false;
 // The temporal pass reads this frame's unfiltered colours and view ray after its taps where they are
 // in L2 by then and would only hold registers across the tap loop (the default path: 91.2 us with them
 // first and 89.1 after at 1920x1080 fp16, 339 and 331 at 3840x2160 bf16, 55.4 and 53.6 at 1366x767), and
@@ -1006,33 +1000,6 @@ __device__ __forceinline__ void temporal_tile( const FrameArgs& a, int bx, int b
         { ( 1.0f - subPix.x ) * ( 1.0f - subPix.y ), subPix.x * ( 1.0f - subPix.y ) },
         { ( 1.0f - subPix.x ) * subPix.y, subPix.x * subPix.y },
     };
-    // FAST: an L2 prefetch of the history rows under the bilinear footprint, so the history
-    // loads that follow the reprojection tests find them on chip
-    if( FAST && kTemporalL2Prefetch && pixPrev.x >= 0 && pixPrev.y >= 0 && pixPrev.x + 1 < u.W && pixPrev.y + 1 < u.H )
-    {
-        const TmaTexel tx = tma_texel( M == MODE_REF ? RGDN_STORAGE_REF : M == MODE_F32 ? RGDN_STORAGE_FP32 : RGDN_STORAGE_FP16 );
-        const int      mb = M == MODE_REF ? 4 : 8;   // moments
-#pragma unroll
-        for( int r = 0; r < 2; r++ )
-        {
-            const size_t q = (size_t)( pixPrev.y + r ) * u.W + pixPrev.x;
-            asm volatile( "prefetch.global.L2 [%0];" ::"l"( static_cast< const char* >( a.diffHistory ) + q * tx.cv ) );
-            asm volatile( "prefetch.global.L2 [%0];" ::"l"( static_cast< const char* >( a.momentsPrev ) + q * mb ) );
-            asm volatile( "prefetch.global.L2 [%0];" ::"l"( static_cast< const char* >( a.histLenPrev ) + q * tx.cv ) );
-            asm volatile( "prefetch.global.L2 [%0];" ::"l"( static_cast< const char* >( a.specAccumPrev ) + q * tx.col ) );
-            asm volatile( "prefetch.global.L2 [%0];" ::"l"( static_cast< const char* >( a.indirAccumPrev ) + q * tx.col ) );
-            if( tx.var ) asm volatile( "prefetch.global.L2 [%0];" ::"l"( a.varHistory + q ) );
-        }
-    }
-    // the surface positions the specular terms read once a tap is accepted: loaded with the
-    // taps (kTemporalEarlySurfPos) or where they are used
-    float4 sp4 = make_float4( 0, 0, 0, 0 ), spp4 = make_float4( 0, 0, 0, 0 );
-    auto   ldSurf = [ & ]() {
-        sp4  = a.surfPos[ i ];
-        spp4 = inside( u, pixPrev.x, pixPrev.y ) ? a.surfPosPrev[ pixPrev.y * u.W + pixPrev.x ] : make_float4( 0, 0, 0, 0 );
-    };
-    if( kTemporalEarlySurfPos ) ldSurf();
-
     float4 histLenDIS     = make_float4( 0, 0, 0, 0 );
     float3 diffPrev       = f3( 0, 0, 0 );
     float2 momentsPrev    = make_float2( 0, 0 );
@@ -1150,7 +1117,8 @@ __device__ __forceinline__ void temporal_tile( const FrameArgs& a, int bx, int b
         const float specHistoryLength   = FAST ? histLenDIS.z * invWS : histLenDIS.z / weightSum;
         const float specHitDistancePrev = FAST ? histLenDIS.w * invWS : histLenDIS.w / weightSum;
 
-        if( !kTemporalEarlySurfPos ) ldSurf();
+        const float4 sp4  = a.surfPos[ i ];
+        const float4 spp4 = inside( u, pixPrev.x, pixPrev.y ) ? a.surfPosPrev[ pixPrev.y * u.W + pixPrev.x ] : make_float4( 0, 0, 0, 0 );
         const float3 surfPos     = f3( sp4.x, sp4.y, sp4.z );
         const float3 surfPosPrev = f3( spp4.x, spp4.y, spp4.z );
         const float nv = fmaxf( 0.0f, X::dot( normal, f3( -rayInfo.x, -rayInfo.y, -rayInfo.z ) ) );
@@ -1548,9 +1516,9 @@ template< int M > __global__ void __launch_bounds__( 256 ) k_variance( const Fra
 // Anti-firefly for the default path (CmAntiFirefly.comp:120-158), the same results as
 // k_antifirefly: min / max are exact in any representation of the stored values, so 16-bit
 // storage clamps on packed half2 / bf16x2 pairs without converting, fp32 on floats, and the
-// shared-exponent storage on half2 pairs, which hold its values exactly. Blocks whose 5x5
-// footprint lies inside the image skip the bounds tests. Every stored colour is non-negative and finite, so the shader's
-// +-1e6 initial extrema never survive the 24 taps and the first tap seeds them.
+// shared-exponent storage on half2 pairs, which hold its values exactly. Every stored colour is
+// non-negative and finite, so the shader's +-1e6 initial extrema never survive the 24 taps and the
+// first tap seeds them.
 // ==========================================================================================
 template< int M > struct AfOps;
 template<> struct AfOps< MODE_F16 >
@@ -1638,43 +1606,6 @@ template<> struct AfOps< MODE_REF > : AfOps< MODE_F16 >
     __device__ static void st( void* p, int i, V v ) { static_cast< uint32_t* >( p )[ i ] = encode( v ); }
 };
 
-template< int M, bool INTERIOR >
-__device__ __forceinline__ void af_signal( const FrameArgs& a, const void* src, void* dst, int px, int py, int i )
-{
-    using O          = AfOps< M >;
-    using V          = typename O::V;
-    const Uniform& u = a.u;
-    V c = O::ld( src, i );
-    if( u.antiFirefly != 0 )
-    {
-        V mn = c, mx = c;
-        bool first = true;
-#pragma unroll
-        for( int oy = -2; oy <= 2; oy++ )
-        {
-#pragma unroll
-            for( int ox = -2; ox <= 2; ox++ )
-            {
-                if( ox == 0 && oy == 0 ) continue;
-                const int qx = px + ox, qy = py + oy;
-                const V   v  = ( INTERIOR || inside( u, qx, qy ) ) ? O::ld( src, qy * u.W + qx ) : O::zero();
-                if( first )
-                {
-                    mn = mx = v;
-                    first = false;
-                }
-                else
-                {
-                    mn = O::mn( mn, v );
-                    mx = O::mx( mx, v );
-                }
-            }
-        }
-        c = O::mn( O::mx( c, mn ), mx );
-    }
-    O::st( dst, i, c );
-}
-
 // The 5x5 clamp (the centre excluded) of a tile of 32 columns x 8 RP rows, blockDim 32 x 8,
 // one signal after the other:
 //   1. the thread of column x and row group ty loads its column's RP + 4 texels (zeros outside
@@ -1683,7 +1614,7 @@ __device__ __forceinline__ void af_signal( const FrameArgs& a, const void* src, 
 //   2. v5 of every column, the two halo columns on each side included, goes to shared memory;
 //   3. the pixel combines its own v4 with v5 of the columns x-2, x-1, x+1, x+2 and clamps its
 //      centre, still in registers.
-// min and max are exact, so this is the 24-tap clamp of af_signal value for value. Shared
+// min and max are exact, so this is the shader's 24-tap clamp value for value. Shared
 // memory carries only the v5 pairs: one 16-byte store and four 16-byte loads per pixel and
 // signal for the packed 16-bit texels.
 template< int M > struct AfOpsRows
@@ -1702,7 +1633,7 @@ template< int M > struct AfShared
     AfPair< M >           v5[ TH ][ RW ];
     typename AfOps< M >::V tile[ TILE ? TILE : 1 ];
 };
-static_assert( sizeof( AfShared< MODE_F32 > ) <= 48 * 1024 && sizeof( AfShared< MODE_F16 > ) <= 48 * 1024,
+static_assert( sizeof( AfShared< MODE_F32 > ) <= 48 * 1024 && sizeof( AfShared< MODE_F16 > ) <= 48 * 1024 && sizeof( AfShared< MODE_REF > ) <= 48 * 1024,
                "the anti-firefly tile must fit static shared memory" );
 
 // Rows r0 - 2 .. r0 + RP + 1 of column x of one signal, zeros outside the image: writes v5 of
@@ -1957,7 +1888,7 @@ template< int M, bool FAST > __device__ __forceinline__ void af_variance_tile( c
             V c = O::ld( a.diffTemp, gy * u.W + gx );
             if( u.antiFirefly != 0 )
             {
-                // the 24-tap clamp of af_signal, zeros outside the image
+                // the shader's 24-tap clamp, zeros outside the image
                 V    mn = c, mx = c;
                 bool first = true;
 #pragma unroll
