@@ -3981,6 +3981,19 @@ template< bool FAST > __device__ __forceinline__ float3 volume_sample_pos( const
     return f3( nx * 0.5f + 0.5f, ny * 0.5f + 0.5f, z );
 }
 
+// fializeScattering (CmScatterAccum.comp:41-95) where it does not sample the volume: fog by depth
+// (SIMPLE), or none
+template< bool FAST > __device__ __forceinline__ float4 scattering_without_volume( const ScatterArgs& a, float depthCb )
+{
+    if( a.enableType == RGDN_VOLUME_ENABLE_SIMPLE )
+    {
+        if( depthCb > MAX_RAY_LENGTH ) return make_float4( 0.0f, 0.0f, 0.0f, 1.0f );
+        const float f = FAST ? ex2_approx( ( -depthCb * a.density ) * 1.44269504088896341f ) : expf( -depthCb * a.density );
+        return make_float4( a.ambient[ 0 ] * ( 1.0f - f ), a.ambient[ 1 ] * ( 1.0f - f ), a.ambient[ 2 ] * ( 1.0f - f ), f );
+    }
+    return make_float4( 0.0f, 0.0f, 0.0f, 1.0f );
+}
+
 // fializeScattering (CmScatterAccum.comp:41-95) at regular pixel (rx, ry); depthCb is
 // DEPTH_WORLD at its checkerboard position
 template< bool FAST >
@@ -4013,13 +4026,7 @@ __device__ __forceinline__ float4 finalize_scattering( const ScatterArgs& a, int
         sp             = f3( sp.x + dx, sp.y + dy, sp.z + ( k * basis.z ) * 0.015625f );
         return volume_trilinear( a.volume, a.nx, a.ny, a.nz, sp );
     }
-    if( a.enableType == RGDN_VOLUME_ENABLE_SIMPLE )
-    {
-        if( depthCb > MAX_RAY_LENGTH ) return make_float4( 0.0f, 0.0f, 0.0f, 1.0f );
-        const float f = FAST ? ex2_approx( ( -depthCb * a.density ) * 1.44269504088896341f ) : expf( -depthCb * a.density );
-        return make_float4( a.ambient[ 0 ] * ( 1.0f - f ), a.ambient[ 1 ] * ( 1.0f - f ), a.ambient[ 2 ] * ( 1.0f - f ), f );
-    }
-    return make_float4( 0.0f, 0.0f, 0.0f, 1.0f );
+    return scattering_without_volume< FAST >( a, depthCb );
 }
 
 // rows 0, 1 and 3 of m * (x, y, z, 1) by fused multiply-adds
@@ -4147,7 +4154,7 @@ __device__ __forceinline__ float4 scatter_pixel( const ScatterArgs& a, int cx, i
         else
         {
             pdl_wait();
-            now = finalize_scattering< true >( a, reg.x, reg.y, depth, inv255 );
+            now = scattering_without_volume< true >( a, depth );
         }
         // two products, as the lerps above: a history of 1 (a reset) gives `now` whatever acc was,
         // and an infinite acc stays infinite
