@@ -3,9 +3,12 @@ the batched kernels, which have one form for every size, bit for bit."""
 import numpy as np
 import pytest
 
+import oracle
 from raytracedgl1_gb300 import _native as N
 from raytracedgl1_gb300.denoiser import Context, Denoiser, Stream, Tonemapping
 from raytracedgl1_gb300.scene import Scene
+from tests import _formats as F
+from tests.test_gpu_parity import run_frames
 
 pytestmark = pytest.mark.gpu
 
@@ -47,3 +50,23 @@ def test_large_frame_equals_batched(mode_name, mode, size):
         assert a.tonemapping()[1] == b.tonemapping()[1]
         a.close()
         b.close()
+
+
+@pytest.mark.parametrize("mode_name,mode", [("ref", N.STORAGE_REF), ("fp32", N.STORAGE_FP32), ("fp16", N.STORAGE_FP16), ("bf16", N.STORAGE_BF16)])
+def test_large_frame_against_the_oracle(mode_name, mode):
+    """The same forms against code that shares nothing with them, to the bounds of test_end_to_end."""
+    W, H = 1502, 1001
+    with Context(0) as ctx:
+        sc = Scene(W, H, seed=71)
+        s, o = Stream(ctx, W, H, mode), oracle.OracleStream(W, H, mode)
+        fi = run_frames(s, o, sc, 3)
+        img = s.image("PRE_FINAL", fi)
+        g = F.decode(s.download("PRE_FINAL", fi), img.format)
+        c = F.decode(o.plane("PRE_FINAL", fi), img.format)
+        err = F.texel_rel_err(g, c, atol=1e-4 * float(np.percentile(c, 99)))
+        if mode == N.STORAGE_FP32:
+            assert err.max() <= 1e-3, f"max rel err {err.max():.3e}"
+        else:
+            assert np.mean(err <= 1e-2) >= 0.99, f"{np.mean(err <= 1e-2):.4f} of pixels within 1e-2"
+            assert F.psnr(g, c) > 50.0
+        s.close()

@@ -1,5 +1,7 @@
 """ProcessScattering of a stream in the reference formats takes the unfused form of the default
 arithmetic: the same bounds against the oracle as the fused form of the other storage modes."""
+import hashlib
+
 import numpy as np
 import pytest
 
@@ -38,3 +40,39 @@ def test_scattering_of_a_reference_stream(vmode, size):
         assert err.max() <= TOL[img.format], f"{name}: max rel err {err.max():.3e}"
         assert np.mean(err > 0) <= 0.02, f"{name}: {np.mean(err > 0):.2%} of texels differ"
     s.close()
+
+
+# SHA-256 of SCATTERING and SCATTERING_HISTORY as the unfused default arithmetic of GB300 gives them
+# for the inputs below (recorded from commit d03ae75, which had no fused form)
+RECORDED = "cfe2b324da0951f6c2b33033258432396b8ebd29968a3ff8c270224eacbb9a5e"
+
+
+def _scattering_digest(storage):
+    W, H = 320, 180
+    rng = np.random.default_rng(17)
+    nx, ny, nz = N.VOLUME_SIZE
+    f16 = lambda v: np.ascontiguousarray(v, np.float32).astype(np.float16).view(np.uint16)
+    planes = {("SCATTER_VOLUME", 0): f16(rng.random((ny * nz, nx, 4), np.float32) * np.float32([0.5, 0.5, 0.5, 0.1])),
+              ("SCATTERING", 1): f16(rng.random((H, W, 4), np.float32)),
+              ("SCATTERING_HISTORY", 1): f16(1 + 4 * rng.random((H, W), np.float32)),
+              ("DEPTH_NDC", 0): (rng.random((H, W), np.float32) * np.float32(0.75) + np.float32(0.125))}
+    for slot in (0, 1):
+        planes["NORMAL", slot] = np.full((H, W), 0x40001000, np.uint32)
+        planes["DEPTH_WORLD", slot] = f16(8 + 0.25 * rng.random((H, W), np.float32))
+    planes["MOTION", 0] = f16((rng.random((H, W, 4), np.float32) - np.float32(0.5)) * np.float32([0.02, 0.02, 0.1, 0]))
+    with Context() as ctx:
+        s = Stream(ctx, W, H, storage)
+        for (name, slot), v in planes.items():
+            s.upload(name, slot, v)
+        Volumetric(s).ProcessScattering(0, _volumetric_params(N.VOLUME_ENABLE_VOLUMETRIC, 5))
+        d = hashlib.sha256(b"".join(s.download(k, 0).tobytes() for k in ("SCATTERING", "SCATTERING_HISTORY"))).hexdigest()
+        s.close()
+    return d
+
+
+def test_reference_stream_keeps_the_unfused_bytes():
+    """The composition of a reference-format stream packs what it reads here into 11- and 10-bit integers:
+    its bytes are those of the unfused arithmetic. The fused form of the other storage modes moves the
+    last bit of some of these texels, so this input tells the two apart."""
+    assert _scattering_digest(N.STORAGE_REF) == RECORDED
+    assert _scattering_digest(N.STORAGE_FP16) != RECORDED
