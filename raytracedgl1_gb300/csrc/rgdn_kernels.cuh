@@ -4144,18 +4144,11 @@ __device__ __forceinline__ float4 scatter_pixel( const ScatterArgs& a, int cx, i
     histOut        = hist;
     if constexpr( FMA )
     {
-        float4 now;
-        if( a.enableType == RGDN_VOLUME_ENABLE_VOLUMETRIC )
-        {
-            const float3 sp = volume_dithered_pos_fast( a, reg.x, reg.y );
-            pdl_wait();
-            now = volume_trilinear_fast( a.volume, sp );
-        }
-        else
-        {
-            pdl_wait();
-            now = scattering_without_volume< true >( a, depth );
-        }
+        const bool volumetric = a.enableType == RGDN_VOLUME_ENABLE_VOLUMETRIC;
+        float3     sp         = f3( 0.0f, 0.0f, 0.0f );
+        if( volumetric ) sp = volume_dithered_pos_fast( a, reg.x, reg.y );
+        pdl_wait();
+        const float4 now = volumetric ? volume_trilinear_fast( a.volume, sp ) : scattering_without_volume< true >( a, depth );
         // two products, as the lerps above: a history of 1 (a reset) gives `now` whatever acc was,
         // and an infinite acc stays infinite
         const float f = rcp_approx( hist ), w = 1.0f - f;
