@@ -34,7 +34,8 @@ CU_SOURCES = ["rgdn_api.cu", "rgdn_mode_ref.cu", "rgdn_mode_f32.cu", "rgdn_mode_
               "rgdn_fast_f16.cu", "rgdn_fast_bf16.cu"]
 # No translation unit lets the compiler contract a*b+c on its own: where the kernels want a
 # fused multiply-add they say so (__fmaf_rn), so every instantiation of a kernel body (the
-# single-frame and the batched kernels) computes the same bits.
+# single-frame and the batched kernels) computes the same bits. The flag does not reach packed FP32x2
+# operations: a __fmul2_rn whose result a __fadd2_rn takes is fused (rgdn_kernels.cuh, P3).
 FMAD_TRUE: set[str] = set()
 HEADERS = ["rgdn_internal.h", "rgdn_kernels.cuh", "rgdn_codec.h", "rgdn_host.h"]
 

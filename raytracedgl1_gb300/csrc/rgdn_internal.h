@@ -53,9 +53,18 @@ struct Uniform
     int      prefetchRows;   // how many rows ahead the large-frame kernels prefetch into L2; 0 = not
 };
 // How far ahead, in pixels (about 2-3 us of a pass): 41 k, 61 k and 82 k measured alike, 8 k 2 %
-// slower and 250 k 4 % slower (the rows are pushed out of L2 again). Frames below
-// PREFETCH_MIN_PIXELS keep in L2 what the pass before wrote: 1366x767 measured 1 % slower with the
-// prefetch on than off, 1920x1080 3.6 % faster.
+// slower and 250 k 4 % slower (the rows are pushed out of L2 again).
+//
+// PREFETCH_MIN_PIXELS is a measured line above which every storage format gains, alone and side by
+// side in a batch; it is not where a frame's planes outgrow L2 (129 MB), which they do at fewer pixels
+// and at different sizes in each format. Us per frame of 4 iterations on GB300, without and with it:
+//              ref              fp32             fp16             bf16
+//   1024x576   150.2  151.6     165.1  164.9     133.7  132.7     134.5  134.5
+//   1366x767   242.3  242.2     282.2  268.4     221.8  216.5     222.3  219.3
+//   1600x900   322.7  318.7     369.8  349.5     296.0  284.1     295.3  286.4
+//   1680x1050  388.2  380.8     439.1  424.5     356.7  338.5     355.3  341.2
+//   2560x1440  756.3  735.7     862.9  843.2     694.0  655.5     689.4  659.9
+// and per batch of four 1920x1080 frames 1691 / 1638 (ref), 1929 / 1764 (fp32), 1544 / 1444 (fp16).
 constexpr int PREFETCH_PIXELS     = 61440;
 constexpr int PREFETCH_MIN_PIXELS = 1500000;
 

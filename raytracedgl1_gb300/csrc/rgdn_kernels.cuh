@@ -822,8 +822,8 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile( "griddep
 __device__ __forceinline__ void pdl_wait() { asm volatile( "griddepcontrol.wait;" ::: "memory" ); }
 
 // L2 prefetch of the rows that the blocks some way ahead in launch order will read. The passes
-// are bound by the latency of loads: once a frame's planes no longer fit the 129 MB L2, each
-// block's first reads of a row go to DRAM. One block in 8 asks for 256 columns of those rows
+// are bound by the latency of loads, and on large frames each block's first reads of a row go to
+// DRAM (Uniform::prefetchRows says which frames). One block in 8 asks for 256 columns of those rows
 // ahead of time, with one bulk prefetch per plane and row (cp.async.bulk.prefetch.L2): no register
 // holds it and it takes next to no issue slots. On GB300 at 1920x1080 fp16 the temporal pass went
 // from 99.3 to 91.8 us, the a-trous iterations from 59.4 / 51.7-52.7 / 73.7 to 55.2 / 51.4-51.6 /
@@ -3518,12 +3518,13 @@ template< int M, bool FAST > __global__ void __launch_bounds__( 256 ) k_prepare_
 // images in PRE_FINAL's format. textureLod with the framebuffers' bilinear clamp-to-edge
 // sampler is evaluated in FP32 (texel centres at +0.5, weights from the fractional position).
 // ==========================================================================================
-// One bloom texel: (r, g) as a pair for the packed FP32x2 operations, b alone. Each packed lane
-// rounds as the scalar operation does. The passes are bound by issue (64 to 67 % of the slots at
-// 2560x1440), so outside the reference formats the weighted sums are fused multiply-adds: one
-// operation and one rounding less for each tap (bloom of 2560x1440 FP16: 120.7 us, 128.5 before;
-// the quad upsample holds 76 registers, 90 before). The reference formats are packed integers
-// whose bytes follow the uncontracted sums.
+// One bloom texel: (r, g) as a pair for the packed FP32x2 operations, b alone. The compiler fuses a
+// packed multiply into the packed add that takes it even under --fmad=false (x w + y a measures as
+// fma( x, w, y a ) for every input), where the scalar b rounds the multiply and the add. The passes
+// are bound by issue (64 to 67 % of the slots at 2560x1440), so outside the reference formats the
+// weighted sums say fused multiply-adds: one operation and one rounding less for each tap (bloom of
+// 2560x1440 FP16: 120.7 us, 128.5 before; the quad upsample holds 76 registers, 90 before). The
+// reference formats are packed integers and keep the sums as they were, and so their codes.
 struct P3
 {
     float2 rg;
