@@ -336,7 +336,7 @@ def load_peaks() -> tuple[float, str]:
 
 def profile_traffic(kernel: str, width: int, height: int, storage: str):
     """DRAM bytes (read + write) per launch of `kernel` from the committed ncu summary
-    (profiles/dram_traffic.md, written by --ncu-traffic from one capture of this build), scaled
+    (profiles/dram_traffic.md, written by --ncu-traffic from one capture, whose build it names), scaled
     from the captured frame size to this one by pixel count. None without a matching row."""
     path = os.path.join(ROOT, "profiles", "dram_traffic.md")
     try:

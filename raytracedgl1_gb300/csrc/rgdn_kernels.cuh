@@ -4162,10 +4162,11 @@ __device__ __forceinline__ float4 scatter_pixel( const ScatterArgs& a, int cx, i
 // One thread per checkerboard pixel. (One thread per pair (cx, cx + W/2), whose regular pixels
 // are neighbours, wrote full sectors but ran 10 % slower: half the warps to hide latency.)
 //
-// Bound by issue (72 % of the slots at 66 % of the warps). On GB300 at 1920x1080 this pass went from
-// 75.1 to 54 us (978 to 720 instructions a pixel: fused multiply-adds and packed lerps, 32-bit
-// offsets, no table of byte / 255 to fill) and the two passes together from 86.2 to 67.3, the volume
-// pass being overlapped. 6 blocks per SM: 5 took 69.8 us, 7 (36 registers) 75.6.
+// Bound by issue (74 % of the slots at 67 % of the warps). On GB300 at 1920x1080 this pass went from
+// 75.4 to 50.7 us (980 to 670 instructions a pixel: fused multiply-adds and packed lerps, 32-bit
+// offsets, no table of byte / 255 to fill) and the two passes together from 86.5 to 67.4, the volume
+// pass being overlapped (a reference-format stream's, unfused: 86.1 to 76.3). 6 blocks per SM: 5
+// measured 4 % slower, 7 (36 registers) 12 %.
 template< int M, bool FAST, bool FMA > __global__ void __launch_bounds__( 256, 6 ) k_scatter_accum( const ScatterArgs a )
 {
     __shared__ float inv255[ FMA ? 1 : 256 ];
